@@ -500,9 +500,10 @@ int sph_stage_times(sph_ctx* ctx, double ms[SPH_NUM_STAGES], int64_t* steps);
 #define SPH_OPT_SMEM_CARVEOUT   2
 /*  SPH_OPT_BLOCK_SIZE: threads per block of the mixed-precision pair passes
  *    (32, 64, 128 (default) or 256).
- *  SPH_OPT_LIST_LEN: neighbour-list entries per lane of those passes: 64,
- *    88 or 120 (default 64 in 2-D, 88 in 3-D).  Each block stages
- *    block/32 x (32 x list + 128) words in shared memory (227 KB at most).
+ *  SPH_OPT_LIST_LEN: size of those passes' candidate buffer: 64, 88 or 120
+ *    (default 64 in 2-D, 88 in 3-D) hold 16, 28 or 40 tiles of 32 candidates
+ *    per warp.  Each block takes block/32 x (192 + 64 x tiles) words of shared
+ *    memory (227 KB at most); what does not fit is walked in pieces.
  *    Both are tuning knobs of the autotuner; results do not depend on them. */
 #define SPH_OPT_BLOCK_SIZE      3
 #define SPH_OPT_LIST_LEN        4

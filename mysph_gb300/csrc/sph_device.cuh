@@ -150,7 +150,7 @@ struct Dev {
 
     float4* posf;
     int precision;     // SPH_PREC_FP64 or SPH_PREC_MIXED
-    int tile_k;        // list length per lane of the tiled (mixed) passes
+    int tile_k;        // candidate buffer of the mixed passes (SPH_OPT_LIST_LEN)
     int tile_tpb;      // threads per block of the tiled (mixed) passes
     int persistent;    // 1: the tiled passes launch only the resident blocks, which stride over the tiles
     int lane_shift;    // log2 of the lanes per target of the FP64 passes A and B (0: one lane)
