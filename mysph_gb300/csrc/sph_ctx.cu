@@ -92,7 +92,8 @@ struct sph_ctx {
     cudaStream_t in_stream = nullptr;
     cudaEvent_t ev_x = nullptr, ev_in = nullptr;
     bool rest_pending = false;
-    // build_hash: the scan of the cell counts runs on aux_stream beside the sort
+    bool inactive = false;      // some real particle has State == -1
+    // build_hash: the scan of the cell counts runs on aux_stream beside a sort
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_keys = nullptr, ev_scan = nullptr;
 };
@@ -352,6 +353,7 @@ int ensure_cells(sph_ctx* ctx, int64_t cells) {
     if (st) { free_list(fresh); return fail(ctx, SPH_E_NOMEM, "cell arrays"); }
     if (d.wstart && ctx->cell_cap > 0)  // keep the wall starts of existing instances
         CK(cudaMemcpyAsync(ws, d.wstart, sizeof(int) * (ctx->cell_cap + 2), cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaMemsetAsync(cc, 0, sizeof(int) * (cap + 2), ctx->stream));   // scan_counts leaves the counts at zero
     CK(cudaStreamSynchronize(ctx->stream));
     free_list(ctx->grid_allocs);
     ctx->grid_allocs = fresh;
@@ -397,25 +399,38 @@ void swap_buffers(Dev& d) {
     std::swap(d.dxp, d.dxp2);
 }
 
-// Cell keys, radix sort, cell starts and the reorder of the real particles
-// (with the half kick when `kick`, for instances past their first step).
+// Cell keys, cell starts and the reorder of the real particles by cell, ties
+// in the order of the last search (with the half kick when `kick`, for
+// instances past their first step).
 // Particles of removed instances sort to the end and are dropped.
 int build_hash(sph_ctx* ctx, bool kick) {
     Dev& d = ctx->d;
     cudaStream_t s = ctx->stream;
     if (d.n_real == 0) { ctx->hash_valid = true; return SPH_OK; }
-    CK(cudaMemsetAsync(d.ccount, 0, sizeof(int) * ((size_t)d.total_cells + 1), s));
-    sph::launch_keys(d, d.n_real, d.xm, d.meta, d.pinst, d.keys, d.vals, d.ccount, s, true);
-    // the cell starts need the counts alone: their scan runs beside the sort
-    CK(cudaEventRecord(ctx->ev_keys, s));
-    CK(cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_keys, 0));
-    cudaError_t e = sph::sort_pairs(d.keys, d.vals, d.keys_s, d.vals_s, d.n_real, ctx->key_bits,
-                                    ctx->sort_scratch, s, &ctx->launches);
-    sph::exclusive_scan_u32((const uint32_t*)d.ccount, (uint32_t*)d.fstart, (int64_t)d.total_cells + 1,
-                            ctx->scan_part, ctx->aux_stream, &ctx->launches);
-    CK(cudaEventRecord(ctx->ev_scan, ctx->aux_stream));
-    CK(cudaStreamWaitEvent(s, ctx->ev_scan, 0));
-    if (e != cudaSuccess) return fail(ctx, SPH_E_CUDA, std::string("radix sort: ") + cudaGetErrorString(e));
+    // Where every real particle is in a cell, the cell counts and the ranks of
+    // their atomics place the particles, and the reorder settles the order
+    // within a cell: five launches.  State == -1 particles and those of removed
+    // systems have no cell (any number of them would share one rank count), so
+    // such a search sorts the keys (15 to 20 launches), with the scan beside it.
+    // Hash stage, sorted and counted: 125 and 34 us on 500,000 particles in
+    // 2-D, 180 and 91 us on 1.69 M in 3-D, 36 and 21 us on 5,000.
+    const bool counted = !ctx->inactive && ctx->pending_remove == 0;
+    sph::launch_keys(d, d.n_real, d.xm, d.meta, d.pinst, d.keys, d.vals, d.ccount, s, true,
+                     counted ? d.keys_s : nullptr);
+    if (counted) {
+        sph::scan_counts(d.ccount, d.fstart, (int64_t)d.total_cells + 1, ctx->scan_part, s, &ctx->launches);
+        sph::launch_place(d, s);
+    } else {
+        CK(cudaEventRecord(ctx->ev_keys, s));
+        CK(cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_keys, 0));
+        cudaError_t e = sph::sort_pairs(d.keys, d.vals, d.keys_s, d.vals_s, d.n_real, ctx->key_bits,
+                                        ctx->sort_scratch, s, &ctx->launches);
+        sph::scan_counts(d.ccount, d.fstart, (int64_t)d.total_cells + 1, ctx->scan_part, ctx->aux_stream,
+                         &ctx->launches);
+        CK(cudaEventRecord(ctx->ev_scan, ctx->aux_stream));
+        CK(cudaStreamWaitEvent(s, ctx->ev_scan, 0));
+        if (e != cudaSuccess) return fail(ctx, SPH_E_CUDA, std::string("radix sort: ") + cudaGetErrorString(e));
+    }
     mark(ctx, 1);
     if (ctx->rest_pending) {
         CK(cudaStreamWaitEvent(s, ctx->ev_in, 0));
@@ -423,14 +438,14 @@ int build_hash(sph_ctx* ctx, bool kick) {
         ++ctx->launches;
         ctx->rest_pending = false;
     }
-    sph::launch_permute(d, kick, s);
+    sph::launch_permute(d, kick, counted, s);
     swap_buffers(d);
     if (!kick) {
         std::swap(d.dvr, d.dvr2);
         std::swap(d.dedt, d.dedt2);
         std::swap(d.dsdt, d.dsdt2);
     }
-    ctx->launches += 3;
+    ctx->launches += counted ? 3 : 2;
     CK(cudaGetLastError());
     if (ctx->pending_remove) {
         d.n_real -= (int)ctx->pending_remove;
@@ -676,7 +691,7 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
     Dev& d = ctx->d;
     const int dim = ctx->prm.dim, D2 = dim * dim;
     const int64_t N = n_r + n_w;
-    bool solid = false;
+    bool solid = false, inactive = false;
     const bool kgc = ctx->prm.flags & SPH_F_KERNEL_CORRECTION;
     const char* kgc_msg = "kernel correction needs every real particle to be a solid "
                           "(Type > 100): for other targets the reference's solve divides 0 by 0";
@@ -697,6 +712,7 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
             }
             hmin = std::min(hmin, B.h);
             hmax = std::max(hmax, B.h);
+            if (b < gen.n_real && B.state == -1) inactive = true;
         }
         st = make_grid_bounds(ctx, P, lo, hi, hmin, hmax, &g);
     } else {
@@ -707,6 +723,8 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
         if (kgc)
             for (int64_t i = 0; i < n_r; ++i)
                 if (type[i] <= 100) return fail(ctx, SPH_E_UNSUPPORTED, kgc_msg);
+        if (state)
+            for (int64_t i = 0; i < n_r; ++i) inactive |= state[i] == -1;
         st = make_grid(ctx, P, N, x, h, &g);
     }
     if (st) return st;
@@ -720,6 +738,8 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
         return fail(ctx, SPH_E_RANGE, "the systems' cell grids exceed 2^31 cells in total");
     if ((st = ensure_cells(ctx, base + g.ncells + 1))) return st;
 
+    // a plain context's only system; a batch keeps the flag once it is set
+    ctx->inactive = inactive || (ctx->batch && ctx->inactive);
     HostInst& hi = ctx->insts[k];
     hi = HostInst{};
     hi.used = true;
@@ -809,17 +829,15 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
                                 (boundary || gen.blocks) ? dt_ + 2 * N : nullptr, dsh, worder, s);
         ++ctx->launches;
         // 2) wall keys -> sort -> wall order; wall cell starts of this instance
-        ce = cudaMemsetAsync(d.ccount + base, 0, sizeof(int) * ((size_t)g.ncells + 1), s); if (ce) goto cuda_fail;
         if (n_w > 0) {
             sph::launch_keys(d, (int)n_w, d.xm + wall_dst, d.meta + wall_dst, d.pinst + wall_dst, d.keys, d.vals,
-                             d.ccount, s, false);
+                             d.ccount, s, false, nullptr);
             ce = sph::sort_pairs(d.keys, d.vals, wkeys, worder, n_w, ctx->key_bits, ctx->sort_scratch, s,
                                  &ctx->launches);
             if (ce) goto cuda_fail;
             ++ctx->launches;
         }
-        sph::exclusive_scan_u32((const uint32_t*)d.ccount + base, (uint32_t*)d.wstart + base, g.ncells + 1,
-                                ctx->scan_part, s, &ctx->launches);
+        sph::scan_counts(d.ccount + base, d.wstart + base, g.ncells + 1, ctx->scan_part, s, &ctx->launches);
         sph::launch_add_offset(d.wstart + base, g.ncells + 1, wall_dst - d.wall_off, s);
         // 3) pack again with the walls in cell order, wall EOS
         sph::launch_pack_upload(d, (int)n_r, (int)n_w, real_dst, wall_dst, k, dx_, dv_, dsc, dsc + N, dsc + 2 * N,
@@ -1066,6 +1084,7 @@ std::vector<StateArray> state_arrays(sph_ctx* ctx) {
     Dev& d = ctx->d;
     const size_t D2 = (size_t)ctx->prm.dim * ctx->prm.dim;
     std::vector<StateArray> a = {
+        // (sph_state_load looks the particles' State up in meta, the fifth)
         {d.xm, sizeof(double4), 0, d.xm2}, {d.vr, sizeof(double4), 0, d.vr2}, {d.eh, sizeof(double4), 0, d.eh2},
         {d.dsp, sizeof(double4), 0, d.dsp2}, {d.meta, sizeof(int4), 0, d.meta2}, {d.pinst, sizeof(int), 0, d.pinst2},
         {d.posf, sizeof(float4), 0}, {d.pa4, sizeof(double4), 0}, {d.tt, sizeof(double) * D2, 0},
@@ -2112,6 +2131,13 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
         hi.n_wall = si.n_wall;
         hi.wall_first = si.wall_first;
         hi.used = si.used != 0;
+    }
+    // the State of the real particles (meta, the fifth array, after four of double4)
+    const unsigned char* meta = in + 4 * sizeof(double4) * (size_t)state_particles(ctx);
+    for (int64_t i = 0; i < h.n_real; ++i) {
+        int4 m;
+        std::memcpy(&m, meta + sizeof(int4) * (size_t)i, sizeof(m));
+        ctx->inactive |= m.w == -1;
     }
     if ((st = state_copy(ctx, const_cast<unsigned char*>(in), false))) return bail(st);
     ctx->uploaded = true;

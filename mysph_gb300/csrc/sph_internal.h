@@ -11,8 +11,11 @@ namespace sph {
 // must hold scan_partials(n) uint32 values.  Adds the launches it issues to
 // *launches.
 int64_t scan_partials(int64_t n);
-void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* partials,
+void exclusive_scan_u32(uint32_t* in, uint32_t* out, int64_t n, uint32_t* partials,
                         cudaStream_t s, int64_t* launches);
+// Exclusive prefix sum of n cell counts into n starts, leaving the counts at
+// zero for the next search (so no step clears them first).
+void scan_counts(int* counts, int* starts, int64_t n, uint32_t* partials, cudaStream_t s, int64_t* launches);
 
 // Stable LSD radix sort of (key, value) pairs; scratch layout and size as
 // sph_sort_scratch_bytes.  Returns a cudaError_t.

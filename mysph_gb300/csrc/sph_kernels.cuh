@@ -9,11 +9,15 @@ namespace sph {
 // Effective force terms of a step, from the flags (singleStep.f90:114-130).
 uint32_t step_terms(const Dev& d);
 
-// Cell keys of n particles; mark_outside sets bit 31 of the values of those
-// outside their grid (the real-particle hash, read by launch_permute).
+// Cell keys and counts of n particles; mark_outside sets bit 31 of the values
+// of those outside their grid (the real-particle hash, read by
+// launch_permute); rank (may be null) receives the places of the particles
+// within their cells for launch_place, which then stands in for a sort.
 void launch_keys(const Dev& d, int n, const double4* xm, const int4* meta, const int* pinst,
-                 uint32_t* keys, uint32_t* vals, int* counts, cudaStream_t s, bool mark_outside);
-void launch_permute(const Dev& d, bool kick, cudaStream_t s);
+                 uint32_t* keys, uint32_t* vals, int* counts, cudaStream_t s, bool mark_outside, uint32_t* rank);
+void launch_place(const Dev& d, cudaStream_t s);
+// counted: vals_s is launch_place's; else the sorted pairs
+void launch_permute(const Dev& d, bool kick, bool counted, cudaStream_t s);
 // Tiled (mixed) passes: dynamic shared memory of a block with `tpb` threads
 // and lists of k entries; the largest dynamic shared memory those kernels
 // may use (cudaFuncAttributeMaxDynamicSharedMemorySize); the default list

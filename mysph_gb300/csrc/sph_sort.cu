@@ -78,30 +78,13 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n, u
     if (threadIdx.x == 0) partials[blockIdx.x] = tot;
 }
 
-// single block: exclusive scan of the per-tile partials (count <= SCAN_TILE)
-__global__ void scan_partials_kernel(uint32_t* partials, int64_t count) {
-    uint32_t v[SCAN_ITEMS];
-    int64_t base = (int64_t)threadIdx.x * SCAN_ITEMS;
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        v[k] = base + k < count ? partials[base + k] : 0;
-        s += v[k];
-    }
-    uint32_t tot;
-    uint32_t run = block_excl_scan(s, &tot);
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < count) partials[base + k] = run;
-        run += v[k];
-    }
-}
-
 // single block, n <= SCAN_THREADS * SCAN1_ITEMS: the whole exclusive scan in
 // one launch (small systems' cell starts, small sort histograms).  In place
 // is allowed: each thread reads its values before the block synchronises.
 constexpr int SCAN1_ITEMS = 16;
-__global__ void __launch_bounds__(SCAN_THREADS) scan_single_kernel(const uint32_t* in, uint32_t* out, int64_t n) {
+// clear: the input is left at zero (scan_counts; then in and out differ).
+__global__ void __launch_bounds__(SCAN_THREADS) scan_single_kernel(uint32_t* in, uint32_t* out, int64_t n,
+                                                                   int clear) {
     const int64_t base = (int64_t)threadIdx.x * SCAN1_ITEMS;
     uint32_t v[SCAN1_ITEMS];
     uint32_t s = 0;
@@ -114,13 +97,20 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_single_kernel(const uint32_
     uint32_t run = block_excl_scan(s, &tot);
 #pragma unroll
     for (int k = 0; k < SCAN1_ITEMS; ++k) {
-        if (base + k < n) out[base + k] = run;
+        if (base + k < n) {
+            out[base + k] = run;
+            if (clear) in[base + k] = 0u;
+        }
         run += v[k];
     }
 }
 
-__global__ void scan_down_kernel(const uint32_t* in, uint32_t* out, int64_t n,
-                                 const uint32_t* __restrict__ partials) {
+// The tile scans.  summed: the partials are their exclusive sums already;
+// else (at most SCAN_TILE tiles) the block adds up those before its own, which
+// saves the launch between.
+__global__ void __launch_bounds__(SCAN_THREADS) scan_down_kernel(uint32_t* in, uint32_t* out, int64_t n,
+                                                                 const uint32_t* __restrict__ partials, int summed,
+                                                                 int clear) {
     int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
     uint32_t s = 0;
@@ -129,11 +119,22 @@ __global__ void scan_down_kernel(const uint32_t* in, uint32_t* out, int64_t n,
         v[k] = base + k < n ? in[base + k] : 0;
         s += v[k];
     }
-    uint32_t tot;
-    uint32_t run = block_excl_scan(s, &tot) + partials[blockIdx.x];
+    uint32_t tot, before;
+    uint32_t run = block_excl_scan(s, &tot);
+    if (summed) {
+        before = partials[blockIdx.x];
+    } else {
+        uint32_t p = 0;
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_THREADS) p += partials[k];
+        block_excl_scan(p, &before);
+    }
+    run += before;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
-        if (base + k < n) out[base + k] = run;
+        if (base + k < n) {
+            out[base + k] = run;
+            if (clear) in[base + k] = 0u;
+        }
         run += v[k];
     }
 }
@@ -350,29 +351,34 @@ cudaError_t noalloc_scratch(cudaStream_t stream, void** out) {
 
 int64_t scan_partials(int64_t n) { return scan_partials_c(n); }
 
-// Three launches per level: tile sums, an exclusive scan of the tile sums
-// (one block when they fit a block's tile, else the same scan one level
-// up, on the partials after this level's), and the tile scans with their
-// offsets.  The scan of level-2 partials runs in place: each thread reads its
-// values before the block synchronises and writes them after.
-void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* partials,
-                        cudaStream_t s, int64_t* launches) {
+// Two launches: tile sums, and the tile scans, whose blocks add up the sums
+// before theirs.  With more tiles than SCAN_TILE, the same scan one level up
+// turns the sums into offsets first (on the partials after this level's; in
+// place: each thread reads its values before the block synchronises and
+// writes them after).
+static void scan_u32(uint32_t* in, uint32_t* out, int64_t n, uint32_t* partials, bool clear, cudaStream_t s,
+                     int64_t* launches) {
     if (n <= 0) return;
     if (n <= (int64_t)SCAN_THREADS * SCAN1_ITEMS) {
-        scan_single_kernel<<<1, SCAN_THREADS, 0, s>>>(in, out, n);
+        scan_single_kernel<<<1, SCAN_THREADS, 0, s>>>(in, out, n, clear ? 1 : 0);
         if (launches) *launches += 1;
         return;
     }
-    int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     scan_reduce_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, n, partials);
-    if (nb <= SCAN_TILE) {
-        scan_partials_kernel<<<1, SCAN_THREADS, 0, s>>>(partials, nb);
-        if (launches) *launches += 1;
-    } else {
-        exclusive_scan_u32(partials, partials, nb, partials + nb, s, launches);
-    }
-    scan_down_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, partials);
+    const bool up = nb > SCAN_TILE;
+    if (up) scan_u32(partials, partials, nb, partials + nb, false, s, launches);
+    scan_down_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, partials, up ? 1 : 0, clear ? 1 : 0);
     if (launches) *launches += 2;
+}
+
+void exclusive_scan_u32(uint32_t* in, uint32_t* out, int64_t n, uint32_t* partials, cudaStream_t s,
+                        int64_t* launches) {
+    scan_u32(in, out, n, partials, false, s, launches);
+}
+
+void scan_counts(int* counts, int* starts, int64_t n, uint32_t* partials, cudaStream_t s, int64_t* launches) {
+    scan_u32(reinterpret_cast<uint32_t*>(counts), reinterpret_cast<uint32_t*>(starts), n, partials, true, s, launches);
 }
 
 // scratch: [keys_alt n][vals_alt n][hist 256*tiles][scan partials]
