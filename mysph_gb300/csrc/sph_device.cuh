@@ -351,9 +351,6 @@ __device__ __forceinline__ KConst make_kconst(int skf, double h) {
 __device__ __forceinline__ double p4(double a) { double a2 = a * a; return a2 * a2; }
 __device__ __forceinline__ double p5(double a) { double a2 = a * a; return (a2 * a2) * a; }
 
-// Cubic-spline gradient factor from r and 1/r (two FMAs per branch, no q).
-// Both branches meet at r = h, so the branch choice near q = 1 does not
-// change the value beyond rounding.
 // a < b (a <= b) for doubles that are +0 or positive: IEEE 754 orders them
 // like their bit patterns, so an integer compare decides it exactly and keeps
 // the compare off the FP64 pipe, the binding unit of the FP64 pair loops.
@@ -364,10 +361,14 @@ __device__ __forceinline__ bool le_pos(double a, double b) {
     return __double_as_longlong(a) <= __double_as_longlong(b);
 }
 
-__device__ __forceinline__ double cubic_g_r(const KConst& k, double r, double rinv) {
-    const double gin = fma(k.B1, r, k.A1);
-    const double gout = fma(k.C1, rinv, fma(k.C2, r, k.C3));
-    return lt_pos(r, k.h) ? gin : gout;   // r >= +0, h > 0
+// Cubic-spline gradient factor.  Both branches meet at r = h, so the branch
+// choice near q = 1 does not change the value beyond rounding.
+// From r^2 and 1/r (no r): r < h: g = A1 + (B1 r^2) / r, else
+// C1 / r + (C2 r^2) / r + C3, both as (P r^2 + Q) / r + R, two FMAs; the
+// branch is chosen on r^2 < h^2.
+__device__ __forceinline__ double cubic_g_r(const KConst& k, double hh, double dr, double rinv) {
+    const bool in = lt_pos(dr, hh);   // hh = h^2; r^2 >= +0
+    return fma(rinv, fma(in ? k.B1 : k.C2, dr, in ? 0.0 : k.C1), in ? k.A1 : k.C3);
 }
 
 // Gradient factor g with dW = g * dx, given q = r/h and 1/r.
@@ -647,19 +648,34 @@ __device__ __forceinline__ void kgc_apply(const double* f, double* g) {
     for (int a = 0; a < DIM; ++a) g[a] = X[a];
 }
 
-// ---- FP64 reciprocal for the pair physics ----------------------------------
-// An FP32 hardware estimate refined by one Newton-Raphson step in FP64,
-// y1 = y0 + y0 (1 - x y0): the relative error after the step is about e0^2
-// for an estimate error e0 (below 1e-7), i.e. about 1e-14, far below the
-// 1e-10 parity bar, at two FP64 operations instead of a full division.
-// Outside the FP32 normal range the FP64 division is used.
-__device__ __forceinline__ double rcp_nr(double x) {
-    const float xf = (float)x;
-    const float ax = fabsf(xf);
-    if (!(ax > 1e-30f && ax < 1e30f)) return 1.0 / x;
-    const double y = (double)(1.0f / xf);
+// ---- FP64 reciprocals for the pair physics ----------------------------------
+// The hardware estimate y0 (about 20 good bits) with one third-order step of
+// Householder's iteration, of which the FP64 pipe, the binding unit of the
+// pair loops, runs five (1/sqrt x) and three (1/x) operations:
+//   1/sqrt x:  e = 1 - x y0^2,  y = y0 + y0 e (1/2 + 3/8 e)
+//   1/x:       e = 1 - x y0,    y = y0 + y0 (e + e^2)
+// The step leaves a relative error of e^3 (e is below 2e-6), under a tenth
+// of an ulp; the rounding of the last operations decides, about one ulp.
+// Arguments outside the normal range (no pair of a real system) take the
+// library's functions.
+__device__ __forceinline__ bool normal_d(double x) {   // positive and normal
+    return (unsigned)((unsigned long long)__double_as_longlong(x) >> 52) - 1u < 0x7feu;
+}
+__device__ __forceinline__ double rsqrt_h(double x) {
+    if (!normal_d(x)) return x == 0.0 ? 0.0 : rsqrt(x);   // 0 for coincident particles
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double rcp_h(double x) {
+    // (the estimate of the largest and smallest exponents leaves the normal range)
+    const unsigned ex = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu;
+    if (ex - 2u > 0x7f9u) return 1.0 / x;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
-    return fma(y, e, y);
+    return fma(y, fma(e, e, e), y);
 }
 
 // ---- warp helpers ----------------------------------------------------------
