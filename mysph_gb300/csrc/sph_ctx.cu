@@ -257,17 +257,18 @@ int ensure_mirrors(sph_ctx* ctx) {
             st |= dalloc(ctx, &d.pd0, N, ctx->allocs); st |= dalloc(ctx, &d.pd1, N, ctx->allocs);
             st |= dalloc(ctx, &d.vd0, N, ctx->allocs); st |= dalloc(ctx, &d.vd1, N, ctx->allocs);
             st |= dalloc(ctx, &d.ed0, N, ctx->allocs); st |= dalloc(ctx, &d.ed1, N, ctx->allocs);
-            st |= dalloc(ctx, &d.ttd, N * D2, ctx->allocs);
+            const int64_t rs = sph::ttd_stride_of(ctx->prm.dim);
+            st |= dalloc(ctx, &d.ttd, N * rs, ctx->allocs);
             if (!st) {
                 cudaMemsetAsync(d.ed1, 0, sizeof(float4) * N, ctx->stream);
-                cudaMemsetAsync(d.ttd, 0, sizeof(float2) * N * D2, ctx->stream);
+                cudaMemsetAsync(d.ttd, 0, sizeof(float2) * N * rs, ctx->stream);
             }
         }
         return st ? SPH_E_NOMEM : SPH_OK;
     }
     if (!d.pr4) {
         st |= dalloc(ctx, &d.pr4, N, ctx->allocs); st |= dalloc(ctx, &d.vf4, N, ctx->allocs);
-        st |= dalloc(ctx, &d.ef4, N, ctx->allocs); st |= dalloc(ctx, &d.pf4, N, ctx->allocs);
+        st |= dalloc(ctx, &d.ef4, N, ctx->allocs);
         st |= dalloc(ctx, &d.tf, N * d.tfs, ctx->allocs);
         if (!st) cudaMemsetAsync(d.tf, 0, sizeof(float) * N * d.tfs, ctx->stream);
     }
@@ -691,7 +692,7 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
     Dev& d = ctx->d;
     const int dim = ctx->prm.dim, D2 = dim * dim;
     const int64_t N = n_r + n_w;
-    bool solid = false, inactive = false;
+    bool solid = false, inactive = false, multi = false;
     const bool kgc = ctx->prm.flags & SPH_F_KERNEL_CORRECTION;
     const char* kgc_msg = "kernel correction needs every real particle to be a solid "
                           "(Type > 100): for other targets the reference's solve divides 0 by 0";
@@ -713,6 +714,7 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
             hmin = std::min(hmin, B.h);
             hmax = std::max(hmax, B.h);
             if (b < gen.n_real && B.state == -1) inactive = true;
+            if (b < gen.n_real && B.type != gen.blocks[0].type) multi = true;
         }
         st = make_grid_bounds(ctx, P, lo, hi, hmin, hmax, &g);
     } else {
@@ -725,6 +727,7 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
                 if (type[i] <= 100) return fail(ctx, SPH_E_UNSUPPORTED, kgc_msg);
         if (state)
             for (int64_t i = 0; i < n_r; ++i) inactive |= state[i] == -1;
+        for (int64_t i = 1; i < n_r; ++i) multi |= type[i] != type[0];
         st = make_grid(ctx, P, N, x, h, &g);
     }
     if (st) return st;
@@ -738,8 +741,9 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
         return fail(ctx, SPH_E_RANGE, "the systems' cell grids exceed 2^31 cells in total");
     if ((st = ensure_cells(ctx, base + g.ncells + 1))) return st;
 
-    // a plain context's only system; a batch keeps the flag once it is set
+    // a plain context's only system; a batch keeps a flag once it is set
     ctx->inactive = inactive || (ctx->batch && ctx->inactive);
+    d.multi_type = multi || (ctx->batch && d.multi_type);
     HostInst& hi = ctx->insts[k];
     hi = HostInst{};
     hi.used = true;
@@ -1071,7 +1075,7 @@ struct StateInst {
     int32_t used, reserved;
 };
 constexpr char kStateMagic[8] = {'S', 'P', 'H', 'S', 'T', 'A', 'T', 'E'};
-constexpr uint32_t kStateVersion = 4;
+constexpr uint32_t kStateVersion = 5;
 
 struct StateArray {
     void* ptr;
@@ -1100,7 +1104,6 @@ std::vector<StateArray> state_arrays(sph_ctx* ctx) {
         a.push_back({d.pr4, sizeof(float4), 0});
         a.push_back({d.vf4, sizeof(float4), 0});
         a.push_back({d.ef4, sizeof(float4), 0});
-        a.push_back({d.pf4, sizeof(float4), 0});
         a.push_back({d.tf, sizeof(float) * d.tfs, 0});
     }
     if (d.sf) {
@@ -2132,12 +2135,15 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
         hi.wall_first = si.wall_first;
         hi.used = si.used != 0;
     }
-    // the State of the real particles (meta, the fifth array, after four of double4)
+    // the State and Type of the real particles (meta, the fifth array, after
+    // four of double4; systems of different Types count as one of several)
     const unsigned char* meta = in + 4 * sizeof(double4) * (size_t)state_particles(ctx);
+    int4 m, m0{};
     for (int64_t i = 0; i < h.n_real; ++i) {
-        int4 m;
         std::memcpy(&m, meta + sizeof(int4) * (size_t)i, sizeof(m));
+        if (i == 0) m0 = m;
         ctx->inactive |= m.w == -1;
+        d.multi_type |= m.x != m0.x;
     }
     if ((st = state_copy(ctx, const_cast<unsigned char*>(in), false))) return bail(st);
     ctx->uploaded = true;

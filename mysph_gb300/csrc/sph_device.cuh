@@ -21,8 +21,8 @@
 //     prev_vr, prev_e, shear_prev: leap-frog "Prev" arrays
 //   FP32 mirrors of the mixed-precision pair passes (SPH_PREC_MIXED):
 //     pr4 float4 (x, y, z relative to the particle's cell origin, cell code)
-//     vf4 float4 (v, rho)   ef4 float4 (h, c, m/rho, m)
-//     pf4 float4 (p/rho^2, p, Type bits, -)   tf/sf float[N*D2]   rf4 float4
+//     vf4 float4 (v, m/rho)   ef4 float4 (h, c, rho, m)
+//     tf/sf float rows of D2 tensor components, m, p/rho^2, Type bits   rf4 float4
 #pragma once
 
 #include <cstdint>
@@ -104,9 +104,14 @@ struct Inst {
     float wall_r0_f;       // wall_r0 in FP32 (external pair terms of the mixed passes)
 };
 
-// Row stride of the FP32 tensor mirrors (tf, sf): Dim^2 floats, padded to 12
-// in 3-D so that a row is three aligned float4 loads (a 2-D row is one).
-__host__ __device__ constexpr int tf_stride_of(int dim) { return dim == 3 ? 12 : dim * dim; }
+// Rows of the FP32 tensor mirrors (tf, sf), read by pass B for every
+// neighbour: the Dim^2 components, then the particle's m, p/rho^2 and Type
+// bits, 12 floats in 3-D and 8 (one unused) in 2-D, so that aligned float4 loads
+// bring all that a receding pair needs beside position and velocity.
+__host__ __device__ constexpr int tf_stride_of(int dim) { return dim == 3 ? 12 : 8; }
+// Rows of the double-float tensor mirror: Dim^2 pairs, in 3-D with p/rho^2
+// after them (ten pairs: five aligned float4 loads).
+__host__ __device__ constexpr int ttd_stride_of(int dim) { return dim == 3 ? 10 : 4; }
 
 struct KRef;
 
@@ -136,6 +141,7 @@ struct Dev {
     int total_cells;          // cells of all instances; key of inactive particles
     int wall_off;             // index of the first wall particle
     int has_solid;
+    int multi_type;           // real particles of one system differ in Type
 
     // double-buffered state (cur)
     double4 *xm, *vr, *eh, *dsp;
@@ -154,12 +160,12 @@ struct Dev {
     int tile_tpb;      // threads per block of the tiled (mixed) passes
     int persistent;    // 1: the tiled passes launch only the resident blocks, which stride over the tiles
     int lane_shift;    // log2 of the lanes per target of the FP64 passes A and B (0: one lane)
-    float4 *pr4, *vf4, *ef4, *pf4, *rf4;
+    float4 *pr4, *vf4, *ef4, *rf4;
     float *tf, *sf;
     // double-float mirrors of the DF64 passes (hi in *0, lo in *1):
     // pd = (x, y, z relative to the grid origin, mass), vd = (v, rho),
     // ed0 = (m/rho hi, lo, h hi, lo), ed1 = (c hi, lo, p/rho^2 hi, lo),
-    // ttd = eta edot / rho^2 (Dim^2 pairs)
+    // ttd = rows of eta edot / rho^2 - p/rho^2 I (ttd_stride_of)
     float4 *pd0, *pd1, *vd0, *vd1, *ed0, *ed1;
     float2* ttd;
     double4* pa4;
@@ -363,12 +369,14 @@ __device__ __forceinline__ bool le_pos(double a, double b) {
 
 // Cubic-spline gradient factor.  Both branches meet at r = h, so the branch
 // choice near q = 1 does not change the value beyond rounding.
-// From r^2 and 1/r (no r): r < h: g = A1 + (B1 r^2) / r, else
-// C1 / r + (C2 r^2) / r + C3, both as (P r^2 + Q) / r + R, two FMAs; the
-// branch is chosen on r^2 < h^2.
-__device__ __forceinline__ double cubic_g_r(const KConst& k, double hh, double dr, double rinv) {
-    const bool in = lt_pos(dr, hh);   // hh = h^2; r^2 >= +0
-    return fma(rinv, fma(in ? k.B1 : k.C2, dr, in ? 0.0 : k.C1), in ? k.A1 : k.C3);
+// r < h: g = A1 + B1 r, else C1 / r + (C2 r + C3): two FMAs on selected
+// constants (the inner branch's 0 / r is exact).  The form without r,
+// (C2 r^2 + C1) / r + C3, saves the product r = r^2 / r as well, but its larger
+// first sum made the error of the pair sums 12 % larger (displaced 3-D
+// lattice against 64-bit mantissas).
+__device__ __forceinline__ double cubic_g_r(const KConst& k, double r, double rinv) {
+    const bool in = lt_pos(r, k.h);   // r >= +0, h > 0
+    return fma(in ? 0.0 : k.C1, rinv, fma(in ? k.B1 : k.C2, r, in ? k.A1 : k.C3));
 }
 
 // Gradient factor g with dW = g * dx, given q = r/h and 1/r.
@@ -512,8 +520,16 @@ __device__ __forceinline__ void write_mirrors(const Dev& d, const Grid& g, int s
     for (int a = 0; a < 3; ++a)
         r[a] = a < d.dim ? (float)(x[a] - (g.lo[a] + (double)c[a] * g.cs)) : 0.0f;
     d.pr4[s] = make_float4(r[0], r[1], r[2], __int_as_float(cell_code(c)));
-    d.vf4[s] = make_float4((float)vr.x, (float)vr.y, (float)vr.z, (float)vr.w);
-    d.ef4[s] = make_float4((float)eh.y, (float)eh.z, (float)eh.w, (float)xm.w);
+    d.vf4[s] = make_float4((float)vr.x, (float)vr.y, (float)vr.z, (float)eh.w);
+    d.ef4[s] = make_float4((float)eh.y, (float)eh.z, (float)vr.w, (float)xm.w);
+}
+
+// m, p/rho^2 and Type of particle s in its row of an FP32 tensor mirror.
+__device__ __forceinline__ void tf_tail(float* base, int d2, int tfs, int s, float m, float P, int type) {
+    float* r = base + (size_t)s * tfs + d2;
+    r[0] = m;
+    r[1] = P;
+    r[2] = __int_as_float(type);
 }
 
 // Kahan-compensated FP32 sum.
@@ -654,8 +670,11 @@ __device__ __forceinline__ void kgc_apply(const double* f, double* g) {
 // pair loops, runs five (1/sqrt x) and three (1/x) operations:
 //   1/sqrt x:  e = 1 - x y0^2,  y = y0 + y0 e (1/2 + 3/8 e)
 //   1/x:       e = 1 - x y0,    y = y0 + y0 (e + e^2)
+// The estimate's low word is zero, so y0^2 is exact and e is rounded once.
 // The step leaves a relative error of e^3 (e is below 2e-6), under a tenth
-// of an ulp; the rounding of the last operations decides, about one ulp.
+// of an ulp; the rounding of the last operation decides.  Against 113-bit
+// values over [1e-105, 1e95], in units of 2^-53: 1/sqrt x 0.421
+// rms and 1.008 at most (the library's the same), 1/x 0.420 and 0.999.
 // Arguments outside the normal range (no pair of a real system) take the
 // library's functions.
 __device__ __forceinline__ bool normal_d(double x) {   // positive and normal
@@ -665,7 +684,7 @@ __device__ __forceinline__ double rsqrt_h(double x) {
     if (!normal_d(x)) return x == 0.0 ? 0.0 : rsqrt(x);   // 0 for coincident particles
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
+    const double e = fma(-x, y * y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 __device__ __forceinline__ double rcp_h(double x) {

@@ -71,19 +71,61 @@ __device__ __forceinline__ DF df_mul_f(const DF& a, float b) {
 // a b + c
 __device__ __forceinline__ DF df_fma(const DF& a, const DF& b, const DF& c) { return df_add(df_mul(a, b), c); }
 
-// 1 / a: an FP32 estimate refined by one Newton step in double-float,
-// y1 = y0 + y0 (1 - a y0).
+// 1 / a and 1 / sqrt(a) (a > 0): an FP32 estimate y0 and the residual of
+// y0, which fused multiply-adds give to FP32 accuracy (its leading part is
+// exact), so the correction y0 (r + r^2) resp. y0 (r / 2 + 3/8 r^2) adds the low
+// half: error about 2^-46, in 8 and 11 FP32 operations (a Newton step in
+// double-float arithmetic took 30 and 38).
 __device__ __forceinline__ DF df_rcp(const DF& a) {
     const float y0 = __frcp_rn(a.hi);
-    const DF r = df_add_f(df_neg(df_mul_f(a, y0)), 1.0f);  // 1 - a y0
-    return df_add_f(df_mul_f(r, y0), y0);
+    const float r = __fmaf_rn(-a.lo, y0, __fmaf_rn(-a.hi, y0, 1.0f));   // 1 - a y0
+    return quick_two_sum(y0, __fmul_rn(y0, __fmaf_rn(r, r, r)));
 }
-// 1 / sqrt(a), a > 0: y1 = y0 + y0 (1 - a y0^2) / 2.
 __device__ __forceinline__ DF df_rsqrt(const DF& a) {
     const float y0 = rsqrtf(a.hi);
-    const DF ay2 = df_mul_f(df_mul_f(a, y0), y0);
-    const DF r = df_add_f(df_neg(ay2), 1.0f);              // 1 - a y0^2
-    return df_add_f(df_mul_f(r, 0.5f * y0), y0);
+    const DF q = two_prod(y0, y0);
+    float r = __fmaf_rn(-a.hi, q.hi, 1.0f);                              // 1 - a y0^2
+    r = __fmaf_rn(-a.hi, q.lo, r);
+    r = __fmaf_rn(-a.lo, q.hi, r);
+    return quick_two_sum(y0, __fmul_rn(y0, __fmaf_rn(__fmul_rn(0.375f, r), r, 0.5f * r)));
+}
+
+// Two double-floats advanced together by the packed FP32 instructions (FADD2 /
+// FMUL2 / FFMA2): per component the operations of the scalar forms above,
+// with subtractions as fused multiply-adds by -1 (which round alike).
+struct DF2 {
+    float2 hi, lo;
+};
+__device__ __forceinline__ DF2 df2(const DF& a, const DF& b) {
+    return DF2{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)};
+}
+__device__ __forceinline__ DF df2_x(const DF2& a) { return DF{a.hi.x, a.lo.x}; }
+__device__ __forceinline__ DF df2_y(const DF2& a) { return DF{a.hi.y, a.lo.y}; }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ DF2 two_sum2(float2 a, float2 b) {
+    const float2 s = __fadd2_rn(a, b);
+    const float2 bb = sub2(s, a);
+    return DF2{s, __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb))};
+}
+__device__ __forceinline__ DF2 df2_add(const DF2& a, const DF2& b) {
+    const DF2 s = two_sum2(a.hi, b.hi);
+    const float2 e = __fadd2_rn(s.lo, __fadd2_rn(a.lo, b.lo));
+    const float2 h = __fadd2_rn(s.hi, e);
+    return DF2{h, sub2(e, sub2(h, s.hi))};
+}
+// a - b
+__device__ __forceinline__ DF2 df2_sub(const DF2& a, const DF2& b) {
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    return df2_add(a, DF2{__fmul2_rn(b.hi, m1), __fmul2_rn(b.lo, m1)});
+}
+__device__ __forceinline__ DF2 df2_mul(const DF2& a, const DF2& b) {
+    const float2 p = __fmul2_rn(a.hi, b.hi);
+    const float2 np = __fmul2_rn(p, make_float2(-1.0f, -1.0f));
+    float2 e = __ffma2_rn(a.hi, b.hi, np);
+    e = __ffma2_rn(a.hi, b.lo, e);
+    e = __ffma2_rn(a.lo, b.hi, e);
+    const float2 h = __fadd2_rn(p, e);
+    return DF2{h, sub2(e, __fadd2_rn(h, np))};
 }
 
 // A compensated accumulator of products and sums (the Dot2 scheme of
@@ -111,6 +153,27 @@ struct DFAcc {
     }
     __device__ __forceinline__ DF value() const { return two_sum(s, c); }
     __device__ __forceinline__ double to_double() const { return (double)s + (double)c; }
+};
+
+// Two of them advanced together.
+struct DFAcc2 {
+    float2 s = make_float2(0.0f, 0.0f), c = make_float2(0.0f, 0.0f);
+    __device__ __forceinline__ void add_prod(const DF2& a, const DF2& b) {
+        const float2 p = __fmul2_rn(a.hi, b.hi);
+        float2 e = __ffma2_rn(a.hi, b.hi, __fmul2_rn(p, make_float2(-1.0f, -1.0f)));
+        e = __ffma2_rn(a.hi, b.lo, e);
+        e = __ffma2_rn(a.lo, b.hi, e);
+        const DF2 t = two_sum2(s, p);
+        s = t.hi;
+        c = __fadd2_rn(c, __fadd2_rn(t.lo, e));
+    }
+    __device__ __forceinline__ void add(const DF2& a) {
+        const DF2 t = two_sum2(s, a.hi);
+        s = t.hi;
+        c = __fadd2_rn(c, __fadd2_rn(t.lo, a.lo));
+    }
+    __device__ __forceinline__ double x() const { return (double)s.x + (double)c.x; }
+    __device__ __forceinline__ double y() const { return (double)s.y + (double)c.y; }
 };
 
 }  // namespace sph
