@@ -253,9 +253,8 @@ int ensure_mirrors(sph_ctx* ctx) {
     const int64_t N = ctx->capacity, D2 = (int64_t)ctx->prm.dim * ctx->prm.dim;
     int st = 0;
     if (ctx->prm.precision == SPH_PREC_DF64) {
-        if (!d.pd0) {
-            st |= dalloc(ctx, &d.pd0, N, ctx->allocs); st |= dalloc(ctx, &d.pd1, N, ctx->allocs);
-            st |= dalloc(ctx, &d.vd0, N, ctx->allocs); st |= dalloc(ctx, &d.vd1, N, ctx->allocs);
+        if (!d.pvd) {
+            st |= dalloc(ctx, &d.pvd, 4 * N, ctx->allocs);
             st |= dalloc(ctx, &d.ed0, N, ctx->allocs); st |= dalloc(ctx, &d.ed1, N, ctx->allocs);
             const int64_t rs = sph::ttd_stride_of(ctx->prm.dim);
             st |= dalloc(ctx, &d.ttd, N * rs, ctx->allocs);
@@ -266,8 +265,8 @@ int ensure_mirrors(sph_ctx* ctx) {
         }
         return st ? SPH_E_NOMEM : SPH_OK;
     }
-    if (!d.pr4) {
-        st |= dalloc(ctx, &d.pr4, N, ctx->allocs); st |= dalloc(ctx, &d.vf4, N, ctx->allocs);
+    if (!d.pv4) {
+        st |= dalloc(ctx, &d.pv4, 2 * N, ctx->allocs);
         st |= dalloc(ctx, &d.ef4, N, ctx->allocs);
         st |= dalloc(ctx, &d.tf, N * d.tfs, ctx->allocs);
         if (!st) cudaMemsetAsync(d.tf, 0, sizeof(float) * N * d.tfs, ctx->stream);
@@ -1100,9 +1099,8 @@ std::vector<StateArray> state_arrays(sph_ctx* ctx) {
         a.push_back({d.dsdt, sizeof(double) * D2, 0});
         a.push_back({d.ras, sizeof(double4), 0});
     }
-    if (d.pr4) {
-        a.push_back({d.pr4, sizeof(float4), 0});
-        a.push_back({d.vf4, sizeof(float4), 0});
+    if (d.pv4) {
+        a.push_back({d.pv4, 2 * sizeof(float4), 0});
         a.push_back({d.ef4, sizeof(float4), 0});
         a.push_back({d.tf, sizeof(float) * d.tfs, 0});
     }
@@ -2008,7 +2006,7 @@ int sph_state_save(sph_ctx* ctx, void* buffer, int64_t size) {
     h.batch = ctx->batch;
     h.max_inst = ctx->max_inst;
     h.has_solid = ctx->d.has_solid;
-    h.mirrors = ctx->d.pr4 != nullptr;
+    h.mirrors = ctx->d.pv4 != nullptr;
     h.dxp = ctx->d.dxp != nullptr;
     h.key_bits = ctx->key_bits;
     h.capacity = ctx->capacity;

@@ -20,9 +20,9 @@
 //     dvr  double4 (dv/dt, drho/dt)  dedt double   dsdt double[N*D2]
 //     prev_vr, prev_e, shear_prev: leap-frog "Prev" arrays
 //   FP32 mirrors of the mixed-precision pair passes (SPH_PREC_MIXED):
-//     pr4 float4 (x, y, z relative to the particle's cell origin, cell code)
-//     vf4 float4 (v, m/rho)   ef4 float4 (h, c, rho, m)
-//     tf/sf float rows of D2 tensor components, m, p/rho^2, Type bits   rf4 float4
+//     pv4 two float4: (x, y, z relative to the particle's cell origin, cell
+//     code), (v, m/rho)   ef4 float4 (h, c, rho, m)   rf4 float4
+//     tf/sf float rows: D2 tensor components, m, p/rho^2, Type bits, in 3-D h, c, rho
 #pragma once
 
 #include <cstdint>
@@ -106,12 +106,12 @@ struct Inst {
 
 // Rows of the FP32 tensor mirrors (tf, sf), read by pass B for every
 // neighbour: the Dim^2 components, then the particle's m, p/rho^2 and Type
-// bits, 12 floats in 3-D and 8 (one unused) in 2-D, so that aligned float4 loads
-// bring all that a receding pair needs beside position and velocity.
-__host__ __device__ constexpr int tf_stride_of(int dim) { return dim == 3 ? 12 : 8; }
-// Rows of the double-float tensor mirror: Dim^2 pairs, in 3-D with p/rho^2
-// after them (ten pairs: five aligned float4 loads).
-__host__ __device__ constexpr int ttd_stride_of(int dim) { return dim == 3 ? 10 : 4; }
+// bits, in 3-D also h, c and rho: 16 floats in 3-D, 8 (one unused) in 2-D, two
+// and one 32-byte loads.
+__host__ __device__ constexpr int tf_stride_of(int dim) { return dim == 3 ? 16 : 8; }
+// Rows of the double-float tensor mirror (ttd): Dim^2 pairs, p/rho^2, h and c,
+// three 32-byte loads in 3-D and two in 2-D.
+__host__ __device__ constexpr int ttd_stride_of(int dim) { return dim == 3 ? 12 : 8; }
 
 struct KRef;
 
@@ -160,13 +160,13 @@ struct Dev {
     int tile_tpb;      // threads per block of the tiled (mixed) passes
     int persistent;    // 1: the tiled passes launch only the resident blocks, which stride over the tiles
     int lane_shift;    // log2 of the lanes per target of the FP64 passes A and B (0: one lane)
-    float4 *pr4, *vf4, *ef4, *rf4;
+    float4 *pv4, *ef4, *rf4;
     float *tf, *sf;
     // double-float mirrors of the DF64 passes (hi in *0, lo in *1):
-    // pd = (x, y, z relative to the grid origin, mass), vd = (v, rho),
+    // pvd = rows of four: (x, y, z relative to the grid origin, mass) hi, lo, (v, rho) hi, lo,
     // ed0 = (m/rho hi, lo, h hi, lo), ed1 = (c hi, lo, p/rho^2 hi, lo),
-    // ttd = rows of eta edot / rho^2 - p/rho^2 I (ttd_stride_of)
-    float4 *pd0, *pd1, *vd0, *vd1, *ed0, *ed1;
+    // ttd = rows of eta edot / rho^2 - p/rho^2 I, p/rho^2, h, c (ttd_stride_of)
+    float4 *pvd, *ed0, *ed1;
     float2* ttd;
     double4* pa4;
     double* tt;
@@ -497,10 +497,11 @@ __device__ __forceinline__ void write_df_mirrors(const Dev& d, const Grid& g, in
     for (int a = 0; a < 3; ++a) r[a] = a < d.dim ? df_from(x[a] - g.lo[a]) : DF{0.0f, 0.0f};
     const DF m = df_from(xm.w), v0 = df_from(vr.x), v1 = df_from(vr.y), v2 = df_from(vr.z), rho = df_from(vr.w);
     const DF V = df_from(eh.w), h = df_from(eh.y), c = df_from(eh.z);
-    d.pd0[s] = make_float4(r[0].hi, r[1].hi, r[2].hi, m.hi);
-    d.pd1[s] = make_float4(r[0].lo, r[1].lo, r[2].lo, m.lo);
-    d.vd0[s] = make_float4(v0.hi, v1.hi, v2.hi, rho.hi);
-    d.vd1[s] = make_float4(v0.lo, v1.lo, v2.lo, rho.lo);
+    float4* row = d.pvd + 4 * (size_t)s;
+    row[0] = make_float4(r[0].hi, r[1].hi, r[2].hi, m.hi);
+    row[1] = make_float4(r[0].lo, r[1].lo, r[2].lo, m.lo);
+    row[2] = make_float4(v0.hi, v1.hi, v2.hi, rho.hi);
+    row[3] = make_float4(v0.lo, v1.lo, v2.lo, rho.lo);
     d.ed0[s] = make_float4(V.hi, V.lo, h.hi, h.lo);
     float4 e1 = d.ed1[s];
     e1.x = c.hi;
@@ -519,17 +520,42 @@ __device__ __forceinline__ void write_mirrors(const Dev& d, const Grid& g, int s
     float r[3];
     for (int a = 0; a < 3; ++a)
         r[a] = a < d.dim ? (float)(x[a] - (g.lo[a] + (double)c[a] * g.cs)) : 0.0f;
-    d.pr4[s] = make_float4(r[0], r[1], r[2], __int_as_float(cell_code(c)));
-    d.vf4[s] = make_float4((float)vr.x, (float)vr.y, (float)vr.z, (float)eh.w);
+    d.pv4[2 * (size_t)s] = make_float4(r[0], r[1], r[2], __int_as_float(cell_code(c)));
+    d.pv4[2 * (size_t)s + 1] = make_float4((float)vr.x, (float)vr.y, (float)vr.z, (float)eh.w);
     d.ef4[s] = make_float4((float)eh.y, (float)eh.z, (float)vr.w, (float)xm.w);
 }
 
-// m, p/rho^2 and Type of particle s in its row of an FP32 tensor mirror.
-__device__ __forceinline__ void tf_tail(float* base, int d2, int tfs, int s, float m, float P, int type) {
-    float* r = base + (size_t)s * tfs + d2;
-    r[0] = m;
+// What follows the tensor in particle s's row of an FP32 tensor mirror (e: its ef4).
+__device__ __forceinline__ void tf_tail(float* base, int dim, int s, const float4& e, float P, int type) {
+    float* r = base + (size_t)s * tf_stride_of(dim) + dim * dim;
+    r[0] = e.w;
     r[1] = P;
     r[2] = __int_as_float(type);
+    if (dim == 3) {
+        r[3] = e.x;
+        r[4] = e.y;
+        r[5] = e.z;
+    }
+}
+
+// 32 bytes in one load (a whole sector; p on a 32-byte boundary).
+struct Row8 {
+    float4 a, b;
+};
+__device__ __forceinline__ Row8 load8(const void* p) {
+    Row8 r;
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+        : "l"(p));
+    return r;
+}
+
+// p/rho^2, h and c of particle s behind the tensor in its ttd row.
+__device__ __forceinline__ void ttd_tail(const Dev& d, int dim, int s, const DF& P, const DF& h, const DF& c) {
+    float2* r = d.ttd + (size_t)s * ttd_stride_of(dim) + dim * dim;
+    r[0] = make_float2(P.hi, P.lo);
+    r[1] = make_float2(h.hi, h.lo);
+    r[2] = make_float2(c.hi, c.lo);
 }
 
 // Kahan-compensated FP32 sum.
