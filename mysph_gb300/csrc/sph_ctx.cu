@@ -418,8 +418,11 @@ int build_hash(sph_ctx* ctx, bool kick) {
     sph::launch_keys(d, d.n_real, d.xm, d.meta, d.pinst, d.keys, d.vals, d.ccount, s, true,
                      counted ? d.keys_s : nullptr);
     if (counted) {
-        sph::scan_counts(d.ccount, d.fstart, (int64_t)d.total_cells + 1, ctx->scan_part, s, &ctx->launches);
-        sph::launch_place(d, s);
+        ++ctx->launches;
+        if (!sph::launch_scan_place(d, (int64_t)d.total_cells + 1, s)) {
+            sph::scan_counts(d.ccount, d.fstart, (int64_t)d.total_cells + 1, ctx->scan_part, s, &ctx->launches);
+            sph::launch_place(d, s);
+        }
     } else {
         CK(cudaEventRecord(ctx->ev_keys, s));
         CK(cudaStreamWaitEvent(ctx->aux_stream, ctx->ev_keys, 0));
@@ -445,7 +448,7 @@ int build_hash(sph_ctx* ctx, bool kick) {
         std::swap(d.dedt, d.dedt2);
         std::swap(d.dsdt, d.dsdt2);
     }
-    ctx->launches += counted ? 3 : 2;
+    ctx->launches += 2;
     CK(cudaGetLastError());
     if (ctx->pending_remove) {
         d.n_real -= (int)ctx->pending_remove;
@@ -554,7 +557,7 @@ int one_step(sph_ctx* ctx) {
     st = run_passes(ctx, sph::step_terms(d), true, false);
     if (st) return st;
     sph::launch_update(d, ctx->stream);
-    ctx->launches += (d.n_real > 0 ? 1 : 0) + (d.n_inst > 0 ? 1 : 0);
+    ctx->launches += sph::update_launches(d);
     mark(ctx, 5);
     CK(cudaGetLastError());
     if (ctx->timing && ++ctx->ev_used == sph_ctx::kPool) flush_timing(ctx);
@@ -921,6 +924,7 @@ int create_ctx(const sph_params* prm, int max_inst, int64_t slots, sph_ctx** out
     st |= dalloc(ctx, &d.keys_s, N, L); st |= dalloc(ctx, &d.vals_s, N, L);
     st |= dalloc(ctx, &d.nneigh, N, L);
     st |= dalloc(ctx, &d.status, 1, L);
+    st |= dalloc(ctx, &d.done, 1, L);
     st |= dalloc(ctx, &d.inst, max_inst, L);
     st |= dalloc(ctx, &ctx->d_mat, (int64_t)max_inst * SPH_MAX_MATERIALS, L);
     st |= dalloc(ctx, &d.cmax, max_inst, L);
@@ -950,6 +954,7 @@ int create_ctx(const sph_params* prm, int max_inst, int64_t slots, sph_ctx** out
     d.lane_shift = 0;
     d.tile_k = sph::default_tile_k(prm->dim);
     cudaMemsetAsync(d.status, 0, sizeof(uint32_t), ctx->stream);
+    cudaMemsetAsync(d.done, 0, sizeof(unsigned), ctx->stream);
     cudaMemsetAsync(d.inst, 0, sizeof(sph::Inst) * max_inst, ctx->stream);
     cudaMemsetAsync(d.cmax, 0, sizeof(unsigned long long) * max_inst, ctx->stream);
     cudaMemsetAsync(d.cres, 0, sizeof(double) * 3 * max_inst, ctx->stream);

@@ -16,6 +16,9 @@ uint32_t step_terms(const Dev& d);
 void launch_keys(const Dev& d, int n, const double4* xm, const int4* meta, const int* pinst,
                  uint32_t* keys, uint32_t* vals, int* counts, cudaStream_t s, bool mark_outside, uint32_t* rank);
 void launch_place(const Dev& d, cudaStream_t s);
+// The scan of `cells` counts and launch_place in one launch, for small systems;
+// false (nothing launched) for others.
+bool launch_scan_place(const Dev& d, int64_t cells, cudaStream_t s);
 // counted: vals_s is launch_place's; else the sorted pairs
 void launch_permute(const Dev& d, bool kick, bool counted, cudaStream_t s);
 // Tiled (mixed) passes: dynamic shared memory of a block with `tpb` threads
@@ -43,8 +46,10 @@ void launch_riemann_density(const Dev& d, cudaStream_t s);
 void launch_pass_a(const Dev& d, bool want_strain, cudaStream_t s);
 void launch_pass_b(const Dev& d, uint32_t terms, bool assemble, cudaStream_t s);
 // leap-frog update of every real particle, then per instance the Courant
-// statistics and the step counter (two launches)
+// statistics and the step counter (update_launches: one launch for a single
+// system, two for a batch)
 void launch_update(const Dev& d, cudaStream_t s);
+int update_launches(const Dev& d);
 void launch_count_neighbors(const Dev& d, int* counts, cudaStream_t s);
 void launch_export_neighbors(const Dev& d, const long long* offsets, int* list, cudaStream_t s);
 void launch_wall_init(const Dev& d, int first, int count, cudaStream_t s);

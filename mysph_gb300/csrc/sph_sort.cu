@@ -88,13 +88,36 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_single_kernel(uint32_t* in,
     const int64_t base = (int64_t)threadIdx.x * SCAN1_ITEMS;
     uint32_t v[SCAN1_ITEMS];
     uint32_t s = 0;
+    // a thread's 16 values in four loads where they lie on 16-byte boundaries
+    const bool wide = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+    const bool quad = wide && base + SCAN1_ITEMS <= n;
+    if (quad) {
 #pragma unroll
-    for (int k = 0; k < SCAN1_ITEMS; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        s += v[k];
+        for (int k = 0; k < SCAN1_ITEMS; k += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(in + base + k);
+            v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN1_ITEMS; ++k) v[k] = base + k < n ? in[base + k] : 0;
     }
+#pragma unroll
+    for (int k = 0; k < SCAN1_ITEMS; ++k) s += v[k];
     uint32_t tot;
     uint32_t run = block_excl_scan(s, &tot);
+    if (quad) {
+#pragma unroll
+        for (int k = 0; k < SCAN1_ITEMS; k += 4) {
+            uint4 q;
+            q.x = run; run += v[k];
+            q.y = run; run += v[k + 1];
+            q.z = run; run += v[k + 2];
+            q.w = run; run += v[k + 3];
+            *reinterpret_cast<uint4*>(out + base + k) = q;
+            if (clear) *reinterpret_cast<uint4*>(in + base + k) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < SCAN1_ITEMS; ++k) {
         if (base + k < n) {
