@@ -952,6 +952,9 @@ int create_ctx(const sph_params* prm, int max_inst, int64_t slots, sph_ctx** out
     d.tile_tpb = 128;
     d.persistent = 0;
     d.lane_shift = 0;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    d.coop_threads = sms * 4 * 2 * 32;
     d.tile_k = sph::default_tile_k(prm->dim);
     cudaMemsetAsync(d.status, 0, sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(d.done, 0, sizeof(unsigned), ctx->stream);
