@@ -159,7 +159,7 @@ struct Dev {
     int tile_k;        // candidate buffer of the mixed passes (SPH_OPT_LIST_LEN)
     int tile_tpb;      // threads per block of the tiled (mixed) passes
     int persistent;    // 1: the tiled passes launch only the resident blocks, which stride over the tiles
-    int coop_threads;  // threads that spread a small system's FP64 pair loops over the device (coop_shift)
+    int coop_a, coop_b;  // threads up to which a small system's FP64 passes spread over the device (coop_shift)
     int lane_shift;    // log2 of the lanes per target of the FP64 passes A and B (0: one lane)
     float4 *pv4, *ef4, *rf4;
     float *tf, *sf;

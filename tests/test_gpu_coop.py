@@ -50,9 +50,9 @@ def beam(dx):
     ("2d_few", lambda: few(dam2(0.05), 37), lambda: dam2(0.006)),
     ("2d_beta", lambda: flagged(dam2(0.03), beta=0.3), lambda: flagged(dam2(0.006), beta=0.3)),
 
-    ("3d_32", lambda: dam3(0.05), lambda: dam3(0.013)),
-    ("3d_8", lambda: dam3(0.03), lambda: dam3(0.013)),
-    ("3d_2", lambda: dam3(0.0185), lambda: dam3(0.013)),
+    ("3d_32", lambda: dam3(0.05), lambda: dam3(0.0115)),
+    ("3d_8", lambda: dam3(0.03), lambda: dam3(0.0115)),
+    ("3d_2", lambda: dam3(0.0185), lambda: dam3(0.0115)),
     ("beam", lambda: beam(1.5e-3), lambda: beam(2.5e-4)),
     ("beam_wide", lambda: beam(4e-4), lambda: beam(2.5e-4)),
 ])
