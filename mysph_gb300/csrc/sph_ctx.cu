@@ -954,9 +954,7 @@ int create_ctx(const sph_params* prm, int max_inst, int64_t slots, sph_ctx** out
     d.lane_shift = 0;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    // warps per scheduler (4 an SM) of 32 threads: see coop_shift
-    d.coop_a = (int)(2.1 * 128 * sms);
-    d.coop_b = (int)((prm->dim == 2 ? 2.6 : 5.4) * 128 * sms);
+    d.coop_unit = sms * 4 * 32;   // four schedulers an SM
     d.tile_k = sph::default_tile_k(prm->dim);
     cudaMemsetAsync(d.status, 0, sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(d.done, 0, sizeof(unsigned), ctx->stream);

@@ -159,7 +159,7 @@ struct Dev {
     int tile_k;        // candidate buffer of the mixed passes (SPH_OPT_LIST_LEN)
     int tile_tpb;      // threads per block of the tiled (mixed) passes
     int persistent;    // 1: the tiled passes launch only the resident blocks, which stride over the tiles
-    int coop_a, coop_b;  // threads up to which a small system's FP64 passes spread over the device (coop_shift)
+    int coop_unit;     // threads of one warp on every scheduler of the device (coop_shift)
     int lane_shift;    // log2 of the lanes per target of the FP64 passes A and B (0: one lane)
     float4 *pv4, *ef4, *rf4;
     float *tf, *sf;
@@ -416,9 +416,9 @@ __device__ __forceinline__ double kernel_g(int skf, const KConst& k, double q, d
 
 // Kernel value W(q).
 __device__ __forceinline__ double kernel_w(int skf, const KConst& k, double q) {
-    if (skf == 1) {
-        if (q >= 0 && q < 1) return k.factor * (((2.0 / 3.0) - q * q) + ((q * q) * q) / 2.0);
-        if (q >= 1 && q <= 2) { double t = 2 - q; return (k.factor * (1.0 / 6.0)) * ((t * t) * t); }
+    if (skf == 1) {   // q >= 0: compares on the bit patterns, off the FP64 pipe
+        if (lt_pos(q, 1.0)) return k.factor * (((2.0 / 3.0) - q * q) + 0.5 * ((q * q) * q));
+        if (le_pos(q, 2.0)) { double t = 2 - q; return (k.factor * (1.0 / 6.0)) * ((t * t) * t); }
         return 0.0;
     } else if (skf == 2) {
         return q < 3.0 ? k.factor * exp(-q * q) : 0.0;
