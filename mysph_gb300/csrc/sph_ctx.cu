@@ -409,7 +409,7 @@ int build_hash(sph_ctx* ctx, bool kick) {
     if (d.n_real == 0) { ctx->hash_valid = true; return SPH_OK; }
     // Where every real particle is in a cell, the cell counts and the ranks of
     // their atomics place the particles, and the reorder settles the order
-    // within a cell: five launches.  State == -1 particles and those of removed
+    // within a cell: three to five launches.  State == -1 particles and those of removed
     // systems have no cell (any number of them would share one rank count), so
     // such a search sorts the keys (15 to 20 launches), with the scan beside it.
     // Hash stage, sorted and counted: 125 and 34 us on 500,000 particles in

@@ -8,7 +8,7 @@ steady-state steps replay as a captured CUDA graph.
 
 The autotuner times a few steps of the actual batch and descends one knob at
 a time: cell size (factor x 2h, a new batch per value), then threads per
-block and neighbour-list length of the mixed pair passes and the shared-
+block and candidate buffer of the mixed pair passes and the shared-
 memory carveout (context options on the same batch).  The best setting per
 (dim, size bucket, system count, precision) goes to a JSON cache.
 """
@@ -28,7 +28,7 @@ from .solver import GpuBatch, GpuSolver
 
 CACHE = Path(os.environ.get("MYSPH_TUNE_CACHE", Path(__file__).resolve().parent / "_build" / "autotune.json"))
 
-# the autotuner's knobs: cell size (x 2h), threads per block and list length
+# the autotuner's knobs: cell size (x 2h), threads per block and candidate buffer
 # of the mixed pair passes, shared-memory carveout of the pair passes
 SPACE = {
     "cell_factor": (1.0, 1.15, 1.3),
