@@ -12,6 +12,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1126,6 +1128,50 @@ std::vector<StateArray> state_arrays(sph_ctx* ctx) {
     return a;
 }
 
+// Payload of a version-4 snapshot in version 5's layout.  The two differ in
+// the FP32 mirrors alone: version 4 held (position, cell code), (v, rho),
+// (h, c, m/rho, m) and (p/rho^2, p, Type) as float4 arrays and tensor rows of
+// 12 floats in 3-D and 4 in 2-D; the values are the same.  Null: no memory or
+// not a payload of this header.
+std::unique_ptr<unsigned char[]> payload_of_v4(const StateHeader& h, const unsigned char* in, int64_t* bytes) {
+    const int64_t np = h.n_real + (h.wall_end - h.wall_off), dim = h.prm.dim, D2 = dim * dim;
+    const int64_t old_row = dim == 3 ? 12 : 4, row = sph::tf_stride_of((int)dim);
+    // what state_arrays has ahead of the mirrors: six double4 (xm, vr, eh, dsp,
+    // pa4, dvr), meta, pinst, posf, tt, dedt
+    int64_t pre = 6 * 32 + 16 + 4 + 16 + 8 * D2 + 8;
+    if (h.has_solid) pre += 24 * D2 + 32;
+    pre = (int64_t)sizeof(StateInst) * h.max_inst + pre * np;
+    const int64_t tens = h.has_solid ? 2 : 1, rf = h.has_solid ? 16 * np : 0;
+    const int64_t rest = h.payload_bytes - pre - (64 + 4 * old_row * tens) * np - rf;
+    if (rest < 0) return nullptr;
+    *bytes = pre + (48 + 4 * row * tens) * np + rf + rest;
+    std::unique_ptr<unsigned char[]> out(new (std::nothrow) unsigned char[(size_t)*bytes]());
+    if (!out) return nullptr;
+    std::memcpy(out.get(), in, (size_t)pre);
+    const unsigned char *pr = in + pre, *vf = pr + 16 * np, *ef = vf + 16 * np, *pf = ef + 16 * np, *tf = pf + 16 * np;
+    unsigned char *pv = out.get() + pre, *e5 = pv + 32 * np, *t5 = e5 + 16 * np;
+    for (int64_t i = 0; i < np; ++i) {
+        float v[4], e[4], q[4], tail[6];
+        std::memcpy(v, vf + 16 * i, 16);
+        std::memcpy(e, ef + 16 * i, 16);
+        std::memcpy(q, pf + 16 * i, 16);
+        std::swap(v[3], e[2]);   // now (v, m/rho) and (h, c, rho, m)
+        std::memcpy(pv + 32 * i, pr + 16 * i, 16);
+        std::memcpy(pv + 32 * i + 16, v, 16);
+        std::memcpy(e5 + 16 * i, e, 16);
+        std::memcpy(tail + 1, q, 4);
+        std::memcpy(tail + 2, q + 2, 4);
+        tail[0] = e[3]; tail[3] = e[0]; tail[4] = e[1]; tail[5] = e[2];
+        for (int64_t k = 0; k < tens; ++k) {
+            unsigned char* r = t5 + 4 * row * (k * np + i);
+            std::memcpy(r, tf + 4 * old_row * (k * np + i), (size_t)(4 * D2));
+            std::memcpy(r + 4 * D2, tail, dim == 3 ? 24 : 12);
+        }
+    }
+    std::memcpy(t5 + 4 * row * tens * np, tf + 4 * old_row * tens * np, (size_t)(rf + rest));
+    return out;
+}
+
 // Live particle ranges: real slots [0, n_real) and wall slots [wall_off, wall_end).
 int64_t state_particles(const sph_ctx* ctx) {
     return (int64_t)ctx->d.n_real + (ctx->wall_end - ctx->d.wall_off);
@@ -2083,7 +2129,7 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
     StateHeader h;
     if (size < (int64_t)sizeof(h)) return SPH_E_INVALID;
     std::memcpy(&h, buffer, sizeof(h));
-    if (std::memcmp(h.magic, kStateMagic, sizeof(h.magic)) != 0 || h.version != kStateVersion ||
+    if (std::memcmp(h.magic, kStateMagic, sizeof(h.magic)) != 0 || (h.version != kStateVersion && h.version != 4u) ||
         h.header_bytes != sizeof(StateHeader) || h.params_bytes != sizeof(sph_params) ||
         h.inst_bytes != sizeof(sph::Inst) || h.material_bytes != sizeof(sph::DevMaterial))
         return SPH_E_INVALID;
@@ -2107,6 +2153,13 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
     }
     int st = check_params(&h.prm);
     if (st) return st;
+    const unsigned char* in = (const unsigned char*)buffer + sizeof(h);
+    std::unique_ptr<unsigned char[]> v5;
+    if (h.version == 4u && h.mirrors) {
+        v5 = payload_of_v4(h, in, &h.payload_bytes);
+        if (!v5) return SPH_E_INVALID;
+        in = v5.get();
+    }
     sph_ctx* ctx = nullptr;
     if ((st = create_ctx(&h.prm, h.max_inst, h.capacity, &ctx))) return st;
     auto bail = [&](int code) { sph_destroy(ctx); return code; };
@@ -2128,7 +2181,6 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
     ctx->step = h.step;
     ctx->time = h.time;
     if (state_payload(ctx) != h.payload_bytes) return bail(SPH_E_INVALID);
-    const unsigned char* in = (const unsigned char*)buffer + sizeof(h);
     for (int k = 0; k < h.max_inst; ++k) {
         StateInst si;
         std::memcpy(&si, in, sizeof(si));
