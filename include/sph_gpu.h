@@ -600,6 +600,25 @@ int sph_probe_fp64_gflops(double* gflops);
  * (0 when they agree). */
 int sph_check_conversions(int64_t n, uint64_t seed, int64_t* mismatches);
 
+/* The arithmetic functions that the passes use in place of CUDA's, evaluated
+ * on the device for n arguments (host arrays; b: the second argument of a
+ * division, else may be null).  out receives the results; the double-float
+ * functions take a as the double-float nearest to it and give their results'
+ * high parts in out and low parts in low (null for the others).  The FP32
+ * functions round their arguments to FP32.  SPH_FN_CUDA_RSQRT is CUDA's own. */
+#define SPH_FN_RSQRT        0   /* 1 / sqrt(a), 0 at 0                       */
+#define SPH_FN_RCP          1   /* 1 / a                                     */
+#define SPH_FN_DIV          2   /* a / b                                     */
+#define SPH_FN_RSQRT_F32    3   /* 1 / sqrt(a), 0 at 0                       */
+#define SPH_FN_DIV_F32      4   /* a / b of the mixed artificial viscosity   */
+#define SPH_FN_RCP_DF       5   /* 1 / a                                     */
+#define SPH_FN_RSQRT_DF     6   /* 1 / sqrt(a), a > 0                        */
+#define SPH_FN_FROM_U32     7   /* the unsigned integer a as a double        */
+#define SPH_FN_NEGATIVE     8   /* 1 where a < 0, else 0                     */
+#define SPH_FN_NAN          9   /* 1 where a is a NaN, else 0                */
+#define SPH_FN_CUDA_RSQRT   10
+int sph_check_function(int32_t fn, int64_t n, const double* a, const double* b, double* out, double* low);
+
 #ifdef __cplusplus
 }
 #endif

@@ -2005,6 +2005,26 @@ int sph_check_conversions(int64_t n, uint64_t seed, int64_t* mismatches) {
     return SPH_OK;
 }
 
+int sph_check_function(int32_t fn, int64_t n, const double* a, const double* b, double* out, double* low) {
+    if (fn < SPH_FN_RSQRT || fn > SPH_FN_CUDA_RSQRT || n < 0 || n > (1 << 24) || !a || !out) return SPH_E_INVALID;
+    if (!b && (fn == SPH_FN_DIV || fn == SPH_FN_DIV_F32)) return SPH_E_INVALID;
+    if (!low && (fn == SPH_FN_RCP_DF || fn == SPH_FN_RSQRT_DF)) return SPH_E_INVALID;
+    if (n == 0) return SPH_OK;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    double* d = nullptr;   // a, b, out, low
+    if (cudaMalloc((void**)&d, 4 * bytes) != cudaSuccess) { cudaGetLastError(); return SPH_E_NOMEM; }
+    cudaError_t e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b ? b : a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        sph::launch_function_check(fn, n, d, d + n, d + 2 * n, d + 3 * n, 0);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && low) e = cudaMemcpy(low, d + 3 * n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? SPH_OK : SPH_E_CUDA;
+}
+
 int sph_probe_fp64_gflops(double* gflops) {
     if (!gflops) return SPH_E_INVALID;
     int dev = 0, sms = 0;

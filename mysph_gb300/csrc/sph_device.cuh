@@ -715,13 +715,13 @@ __device__ __forceinline__ void kgc_apply(const double* f, double* g) {
 // pair loops, runs five (1/sqrt x) and three (1/x) operations:
 //   1/sqrt x:  e = 1 - x y0^2,  y = y0 + y0 e (1/2 + 3/8 e)
 //   1/x:       e = 1 - x y0,    y = y0 + y0 (e + e^2)
-// The estimate's low word is zero, so y0^2 is exact and e is rounded once.
-// The step leaves a relative error of e^3 (e is below 2e-6), under a tenth
-// of an ulp; the rounding of the last operation decides.  Against 113-bit
-// values over [1e-105, 1e95], in units of 2^-53: 1/sqrt x 0.421
-// rms and 1.008 at most (the library's the same), 1/x 0.420 and 0.999.
-// Arguments outside the normal range (no pair of a real system) take the
-// library's functions.
+// (the expansions of (1 - e)^(-1/2) and (1 - e)^(-1) to e^2).  The estimates
+// have 32 zero bits at their low end, so y0^2 is exact and e is rounded once.
+// The step leaves 5/16 e^3 and e^3 (e is below 2e-6), a few hundredths of
+// 2^-53; the rounding of the last operation decides, so a result is within
+// 1.04 x 2^-53 of the exact one, relatively (checked against exact arithmetic
+// over the whole range).  Arguments outside the normal range (no pair of a
+// real system) take CUDA's functions.
 __device__ __forceinline__ bool normal_d(double x) {   // positive and normal
     return (unsigned)((unsigned long long)__double_as_longlong(x) >> 52) - 1u < 0x7feu;
 }
@@ -742,9 +742,10 @@ __device__ __forceinline__ double rcp_h(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
-// n / d: n times that reciprocal, and the residual's correction (within a
-// hair of half an ulp), six operations instead of the library's ten and its
-// branches; what is zero, subnormal, infinite or NaN goes to the division.
+// n / d: n times that reciprocal and one correction by the residual (Markstein's
+// final step of a division): the residual n - q d is exact, so the result is
+// within 2^-53 and some 1e-16 of that.  Operands that are zero, subnormal,
+// infinite, NaN or far from 1 take the division.
 __device__ __forceinline__ double div_h(double n, double d) {
     const unsigned en = (unsigned)((unsigned long long)__double_as_longlong(n) >> 52) & 0x7ffu;
     const unsigned ed = (unsigned)((unsigned long long)__double_as_longlong(d) >> 52) & 0x7ffu;

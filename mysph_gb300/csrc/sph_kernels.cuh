@@ -79,5 +79,8 @@ void set_pass_carveout(int percent);
 void launch_add_offset(int* a, int64_t n, int off, cudaStream_t s);
 void launch_fp64_probe(double* sink, int iters, int blocks, cudaStream_t s);
 void launch_conversion_check(int64_t n, uint64_t seed, unsigned long long* bad, cudaStream_t s);
+// out[k] (and low[k]) = function fn (SPH_FN_*) of a[k] and b[k].
+void launch_function_check(int fn, int64_t n, const double* a, const double* b, double* out, double* low,
+                           cudaStream_t s);
 
 }  // namespace sph
