@@ -83,10 +83,11 @@ __device__ __forceinline__ DF df_rcp(const DF& a) {
 }
 __device__ __forceinline__ DF df_rsqrt(const DF& a) {
     const float y0 = rsqrtf(a.hi);
-    const DF q = two_prod(y0, y0);
-    float r = __fmaf_rn(-a.hi, q.hi, 1.0f);                              // 1 - a y0^2
-    r = __fmaf_rn(-a.hi, q.lo, r);
-    r = __fmaf_rn(-a.lo, q.hi, r);
+    // 1 - (a y0) y0: a y0 is about sqrt(a), so it and its low half stay normal
+    // over FP32's whole range, which y0^2 does not
+    const float z = __fmul_rn(a.hi, y0);
+    const float zl = __fmaf_rn(a.lo, y0, __fmaf_rn(a.hi, y0, -z));
+    const float r = __fmaf_rn(-zl, y0, __fmaf_rn(-z, y0, 1.0f));
     return quick_two_sum(y0, __fmul_rn(y0, __fmaf_rn(__fmul_rn(0.375f, r), r, 0.5f * r)));
 }
 
