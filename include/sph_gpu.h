@@ -526,6 +526,11 @@ int sph_stage_times(sph_ctx* ctx, double ms[SPH_NUM_STAGES], int64_t* steps);
 #define SPH_OPT_LANES           6
 int sph_set_option(sph_ctx* ctx, int32_t option, double value);
 
+/* The SPH_OPT_SMEM_CARVEOUT preference (-1: driver default) that the kernels
+ * of the next step's passes A and B carry, for the context's present size,
+ * precision and options. */
+int sph_get_carveout(sph_ctx* ctx, int32_t percent[2]);
+
 /* Number of kernel launches issued by this context since creation. */
 int sph_launch_count(sph_ctx* ctx, int64_t* count);
 

@@ -69,6 +69,7 @@ SIGNATURES = {
     "sph_enable_stage_timing": (C.c_int, [ctxp, C.c_int32]),
     "sph_stage_times": (C.c_int, [ctxp, dp, i64p]),
     "sph_set_option": (C.c_int, [ctxp, C.c_int32, C.c_double]),
+    "sph_get_carveout": (C.c_int, [ctxp, ip]),
     "sph_launch_count": (C.c_int, [ctxp, i64p]),
     "sph_device_bytes": (C.c_int, [ctxp, i64p]),
     "sph_get_params": (C.c_int, [ctxp, C.POINTER(P.SphParams)]),

@@ -1970,6 +1970,14 @@ int sph_set_option(sph_ctx* ctx, int32_t option, double value) {
     }
 }
 
+int sph_get_carveout(sph_ctx* ctx, int32_t percent[2]) {
+    if (!percent) return SPH_E_INVALID;
+    const int st = need(ctx, false);
+    if (st) return st;
+    if (sph::pass_carveout(ctx->d, percent)) return fail(ctx, SPH_E_CUDA, "kernel attributes");
+    return SPH_OK;
+}
+
 int sph_launch_count(sph_ctx* ctx, int64_t* count) {
     if (!ctx || !count) return SPH_E_INVALID;
     *count = ctx->launches;

@@ -76,6 +76,8 @@ void launch_host_state(const Dev& d, int mode, double* stage, cudaStream_t s);
 int launch_energy(const Dev& d, int inst, double* part, double* out, cudaStream_t s);
 // carveout in percent (-1: default) for the pair-pass kernels
 void set_pass_carveout(int percent);
+// The preference of the kernels that the next passes A and B of a step run.
+int pass_carveout(const Dev& d, int percent[2]);
 void launch_add_offset(int* a, int64_t n, int off, cudaStream_t s);
 void launch_fp64_probe(double* sink, int iters, int blocks, cudaStream_t s);
 void launch_conversion_check(int64_t n, uint64_t seed, unsigned long long* bad, cudaStream_t s);

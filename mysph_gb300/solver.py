@@ -268,6 +268,12 @@ class GpuSolver:
         self.set_option(P.OPT_LANES, best)
         return best
 
+    def carveout(self) -> tuple[int, int]:
+        """The shared-memory carveout that passes A and B carry (sph_get_carveout)."""
+        out = (C.c_int32 * 2)()
+        self._call("sph_get_carveout", out)
+        return out[0], out[1]
+
     def launch_count(self) -> int:
         n = C.c_int64()
         self._call("sph_launch_count", C.byref(n))
