@@ -35,6 +35,8 @@ struct HostInst {
     int64_t n_real = 0, n_wall = 0;
     int64_t wall_first = 0; // slot of its first wall
     bool used = false;      // slot taken (active or removed-but-not-compacted)
+    bool inactive = false;    // some real particle has State == -1
+    bool multi_type = false;  // its real particles differ in Type
 };
 
 }  // namespace
@@ -94,7 +96,7 @@ struct sph_ctx {
     cudaStream_t in_stream = nullptr;
     cudaEvent_t ev_x = nullptr, ev_in = nullptr;
     bool rest_pending = false;
-    bool inactive = false;      // some real particle has State == -1
+    bool inactive = false;      // a system in use has one with State == -1 (derive_flags)
     // build_hash: the scan of the cell counts runs on aux_stream beside a sort
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t ev_keys = nullptr, ev_scan = nullptr;
@@ -247,6 +249,17 @@ int pull_instances(sph_ctx* ctx) {
         ctx->insts[k].I.time = tab[k].time;
     }
     return SPH_OK;
+}
+
+// What any system of the context asks of the search and of pass B.
+void derive_flags(sph_ctx* ctx) {
+    ctx->inactive = false;
+    ctx->d.multi_type = 0;
+    for (const HostInst& h : ctx->insts) {
+        if (!h.used) continue;
+        ctx->inactive |= h.inactive;
+        ctx->d.multi_type |= h.multi_type;
+    }
 }
 
 // FP32 mirrors of the mixed-precision passes (allocated on first use).
@@ -745,12 +758,12 @@ int add_instance(sph_ctx* ctx, int k, const sph_params& P, int64_t n_r, int64_t 
         return fail(ctx, SPH_E_RANGE, "the systems' cell grids exceed 2^31 cells in total");
     if ((st = ensure_cells(ctx, base + g.ncells + 1))) return st;
 
-    // a plain context's only system; a batch keeps a flag once it is set
-    ctx->inactive = inactive || (ctx->batch && ctx->inactive);
-    d.multi_type = multi || (ctx->batch && d.multi_type);
     HostInst& hi = ctx->insts[k];
     hi = HostInst{};
     hi.used = true;
+    hi.inactive = inactive;
+    hi.multi_type = multi;
+    derive_flags(ctx);
     hi.prm = P;
     hi.n_real = n_r;
     hi.n_wall = n_w;
@@ -1097,7 +1110,7 @@ std::vector<StateArray> state_arrays(sph_ctx* ctx) {
     Dev& d = ctx->d;
     const size_t D2 = (size_t)ctx->prm.dim * ctx->prm.dim;
     std::vector<StateArray> a = {
-        // (sph_state_load looks the particles' State up in meta, the fifth)
+        // (sph_state_load looks the particles' State, Type and system up in meta and pinst)
         {d.xm, sizeof(double4), 0, d.xm2}, {d.vr, sizeof(double4), 0, d.vr2}, {d.eh, sizeof(double4), 0, d.eh2},
         {d.dsp, sizeof(double4), 0, d.dsp2}, {d.meta, sizeof(int4), 0, d.meta2}, {d.pinst, sizeof(int), 0, d.pinst2},
         {d.posf, sizeof(float4), 0}, {d.pa4, sizeof(double4), 0}, {d.tt, sizeof(double) * D2, 0},
@@ -1778,6 +1791,7 @@ int sph_batch_add(sph_ctx* ctx, const sph_params* prm, int64_t n_real, int64_t n
     st = add_instance(ctx, k, *prm, n_real, n_wall, x, v, mass, rho, p, e, c, h, type, state, boundary, shear);
     if (st) {
         ctx->insts[k].used = false;
+        derive_flags(ctx);
         return st;
     }
     *inst = k;
@@ -1816,6 +1830,7 @@ int sph_batch_add_blocks(sph_ctx* ctx, const sph_params* prm, int32_t n_blocks, 
                       nullptr, nullptr, nullptr, nullptr, nullptr, src);
     if (st) {
         ctx->insts[k].used = false;
+        derive_flags(ctx);
         return st;
     }
     *inst = k;
@@ -1834,6 +1849,7 @@ int sph_batch_remove(sph_ctx* ctx, int32_t inst) {
     // its walls and cells stay until the slot is reused or the batch compacts
     ctx->pending_remove += h.n_real;
     h.used = false;
+    derive_flags(ctx);
     ctx->hash_valid = false;
     return SPH_OK;
 }
@@ -2221,16 +2237,23 @@ int sph_state_load(const void* buffer, int64_t size, sph_ctx** out) {
         hi.wall_first = si.wall_first;
         hi.used = si.used != 0;
     }
-    // the State and Type of the real particles (meta, the fifth array, after
-    // four of double4; systems of different Types count as one of several)
+    // the State and Type of each system's real particles (meta and pinst, the
+    // fifth and sixth arrays, after four of double4)
     const unsigned char* meta = in + 4 * sizeof(double4) * (size_t)state_particles(ctx);
-    int4 m, m0{};
+    const unsigned char* pinst = meta + sizeof(int4) * (size_t)state_particles(ctx);
+    std::vector<int> type_of(h.max_inst, 0);
+    std::vector<char> seen(h.max_inst, 0);
     for (int64_t i = 0; i < h.n_real; ++i) {
-        std::memcpy(&m, meta + sizeof(int4) * (size_t)i, sizeof(m));
-        if (i == 0) m0 = m;
-        ctx->inactive |= m.w == -1;
-        d.multi_type |= m.x != m0.x;
+        int4 m;
+        int k;
+        std::memcpy(&m, meta + sizeof(m) * (size_t)i, sizeof(m));
+        std::memcpy(&k, pinst + sizeof(k) * (size_t)i, sizeof(k));
+        if (k < 0 || k >= h.max_inst) return bail(SPH_E_INVALID);
+        if (!seen[k]) { seen[k] = 1; type_of[k] = m.x; }
+        ctx->insts[k].inactive |= m.w == -1;
+        ctx->insts[k].multi_type |= m.x != type_of[k];
     }
+    derive_flags(ctx);
     if ((st = state_copy(ctx, const_cast<unsigned char*>(in), false))) return bail(st);
     ctx->uploaded = true;
     ctx->hash_valid = false;
