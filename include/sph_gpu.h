@@ -277,7 +277,7 @@ int sph_info(sph_ctx* ctx, int64_t* n_real, int64_t* n_wall, int64_t* step,
  * host arrays (n_real entries, uploaded order).  They mirror the module
  * procedures of the reference one by one. */
 
-/* Build the cell hash (keys, radix sort, cell ranges) over all particles.
+/* Build the cell hash (keys, cell ranges, order by cell) over all particles.
  * Replaces BGGS's grid (src/NNPS/asymmetricSearch.f90:49-158). */
 int sph_nnps(sph_ctx* ctx);
 
@@ -481,7 +481,7 @@ int sph_get_stream(sph_ctx* ctx, void** stream);
  * each stage on the context stream.  sph_stage_times returns the summed
  * milliseconds of each stage since the last reset (SPH_STAGE_* order) and
  * the number of steps they cover. */
-#define SPH_STAGE_HASH     0   /* cell keys + radix sort + cell ranges     */
+#define SPH_STAGE_HASH     0   /* cell keys, cell ranges, order by cell    */
 #define SPH_STAGE_PERMUTE  1   /* reorder state + half-kick                */
 #define SPH_STAGE_PASS_A   2   /* density / divergence / strain rate + EOS */
 #define SPH_STAGE_PASS_B   3   /* forces                                   */
@@ -499,11 +499,11 @@ int sph_stage_times(sph_ctx* ctx, double ms[SPH_NUM_STAGES], int64_t* steps);
 #define SPH_OPT_GRAPHS          1
 #define SPH_OPT_SMEM_CARVEOUT   2
 /*  SPH_OPT_BLOCK_SIZE: threads per block of the mixed-precision pair passes
- *    (32, 64, 128 (default) or 256).
+ *    (32, 64 or 128 (default)).
  *  SPH_OPT_LIST_LEN: size of those passes' candidate buffer: 64, 88 or 120
  *    (default 64 in 2-D, 88 in 3-D) hold 16, 28 or 40 tiles of 32 candidates
  *    per warp.  Each block takes block/32 x (192 + 64 x tiles) words of shared
- *    memory (227 KB at most); what does not fit is walked in pieces.
+ *    memory (43 KB at most); what does not fit is walked in pieces.
  *    Both are tuning knobs of the autotuner; results do not depend on them. */
 #define SPH_OPT_BLOCK_SIZE      3
 #define SPH_OPT_LIST_LEN        4

@@ -1958,10 +1958,6 @@ int sph_set_option(sph_ctx* ctx, int32_t option, double value) {
             if (v != 64 && v != 88 && v != 120) return fail(ctx, SPH_E_INVALID, "list length: 64, 88 or 120");
             k = v;
         }
-        const size_t smem = sph::tiled_smem_bytes(tpb, k);
-        if (smem > 227 * 1024) return fail(ctx, SPH_E_INVALID, "block size x list length needs more than 227 KB");
-        if (smem > 48 * 1024 && sph::set_tiled_smem_limit(smem) != 0)
-            return fail(ctx, SPH_E_CUDA, "cannot raise the dynamic shared memory limit");
         ctx->d.tile_tpb = tpb;
         ctx->d.tile_k = k;
         drop_graph(ctx);

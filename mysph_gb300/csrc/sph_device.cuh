@@ -165,8 +165,9 @@ struct Dev {
     float *tf, *sf;
     // double-float mirrors of the DF64 passes (hi in *0, lo in *1):
     // pvd = rows of four: (x, y, z relative to the grid origin, mass) hi, lo, (v, rho) hi, lo,
-    // ed0 = (m/rho hi, lo, h hi, lo), ed1 = (c hi, lo, p/rho^2 hi, lo),
-    // ttd = rows of eta edot / rho^2 - p/rho^2 I, p/rho^2, h, c (ttd_stride_of)
+    // ttd = rows of eta edot / rho^2 - p/rho^2 I, p/rho^2, h, c (ttd_stride_of),
+    // ed0 = (m/rho hi, lo, h hi, lo), ed1 = (c hi, lo, p/rho^2 hi, lo); of the
+    // last two the passes read m/rho alone, sph_set_field the rest for the rows
     float4 *pvd, *ed0, *ed1;
     float2* ttd;
     double4* pa4;

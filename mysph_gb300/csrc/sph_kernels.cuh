@@ -22,11 +22,8 @@ bool launch_scan_place(const Dev& d, int64_t cells, cudaStream_t s);
 // counted: vals_s is launch_place's; else the sorted pairs
 void launch_permute(const Dev& d, bool kick, bool counted, cudaStream_t s);
 // Tiled (mixed) passes: dynamic shared memory of a block with `tpb` threads
-// and lists of k entries; the largest dynamic shared memory those kernels
-// may use (cudaFuncAttributeMaxDynamicSharedMemorySize); the default list
-// length.
+// and the candidate buffer of SPH_OPT_LIST_LEN = k; the default of that option.
 size_t tiled_smem_bytes(int tpb, int k);
-int set_tiled_smem_limit(size_t bytes);
 int default_tile_k(int dim);
 // Generated blocks into the staging columns of an upload (see sph_block).
 void launch_generate_blocks(const sph_block* blocks, const int64_t* start, int nb, int dim, int64_t N,
